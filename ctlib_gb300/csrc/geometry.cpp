@@ -52,6 +52,7 @@ bool build(const double* o, int n, HostGeom& g, std::string& err) {
   g.fbt.assign((size_t)V * D, 1.0);
   g.lp.assign((size_t)V * L * 2, 0.0);
   g.inv.assign((size_t)V * 5, 0.0);
+  g.slope.assign(V, 0.0);
 
   const double PI = std::acos(-1.0);
   const double x0 = -(double)width / 2 * (double)dImg;   // left image edge (src/fan_ed_kernel.cu:107)
@@ -73,6 +74,7 @@ bool build(const double* o, int n, HostGeom& g, std::string& err) {
     const bool flip = e2 >= 3 && e2 < 7;
     const double c = std::cos(ang), s = std::sin(ang);
     g.flags[v] = (xb ? 1 : 0) | (flip ? 2 : 0);
+    if (g.scan == kPara) g.slope[v] = xb ? s / c : c / s;
     const double sx = -s * (double)s2r, sy = c * (double)s2r;
     g.src[2 * v] = sx; g.src[2 * v + 1] = sy;
     if (g.scan != kPara) {
@@ -214,6 +216,41 @@ bool build(const double* o, int n, HostGeom& g, std::string& err) {
 }
 
 }  // namespace
+
+CellWalk cell_walk(const HostGeom& g, int v, int d) {
+  const bool xb = g.flags[v] & 1;
+  const int nl = xb ? g.H : g.W, N = xb ? g.W : g.H;
+  const double h = g.dImg, edge = xb ? g.x0 : g.y0;
+  // line l lies at p0 + l * step across the walk (rows go down, columns right)
+  const double p0 = xb ? (g.height / 2 - 0.5) * h : (0.5 - g.width / 2) * h, step = xb ? -1.0 : 1.0;
+  const double across = xb ? g.src[2 * v + 1] : g.src[2 * v], along = xb ? g.src[2 * v] : g.src[2 * v + 1];
+  auto ray = [&](double b, double& u0, double& du) {
+    // position along the walk at line position p: b + t p with t = (along - b) /
+    // across for a fan's ray through the source, -slope for a parallel one
+    const double t = g.scan == kPara ? -g.slope[v] : (along - b) / across;
+    u0 = (b + t * p0 - edge) / h;
+    du = t * step;
+  };
+  CellWalk c;
+  double u1, du1;
+  const size_t b = (size_t)v * (g.D + 1) + d;
+  ray(g.db[b], c.u0, c.du);
+  ray(g.db[b + 1], u1, du1);
+  c.w0 = u1 - c.u0;
+  c.dw = du1 - c.du;
+  double lo = 0, hi = nl - 1;
+  // lines with a + s l > 0
+  auto keep = [&](double a, double s) {
+    if (s > 0) lo = std::fmax(lo, std::floor(-a / s) - 1);
+    else if (s < 0) hi = std::fmin(hi, std::ceil(-a / s) + 1);
+    else if (!(a > 0)) hi = -1;
+  };
+  keep(u1, du1);         // the upper boundary right of the image's left edge
+  keep(N - c.u0, -c.du); // the lower boundary left of its right edge
+  if (lo <= hi) { c.first = (int)lo; c.last = (int)hi; }
+  else { c.first = 65535; c.last = 0; }
+  return c;
+}
 
 // RL kernel value at integer offset x for tap spacing d (src/fan_ed_kernel.cu:926-943)
 static double rl_tap(long x, double d) {

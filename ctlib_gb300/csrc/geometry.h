@@ -44,7 +44,20 @@ struct HostGeom {
   double dfilt = 0.0;          // tap spacing of the ramp filter (virtual bin, or dDet)
   std::vector<double> options; // the options vector the geometry was built from
   double x0 = 0, y0 = 0;       // left image edge x, bottom image edge y
+  std::vector<double> slope;   // V: parallel beams, d(axis coordinate)/d(line position) of a ray
 };
+
+// A detector-cell boundary is a straight ray, so its position on the image
+// lines of a view, in pixel-edge units, is linear in the line index: u(l) = u0 +
+// du * l. Likewise the cell's width w(l) = w0 + dw * l in pixels.
+struct CellWalk {
+  double u0, du;  // lower boundary
+  double w0, dw;  // width
+  // lines first .. last of the view are the only ones on which the cell meets
+  // the image (one line of margin on each side); first > last: none
+  int first, last;
+};
+CellWalk cell_walk(const HostGeom& g, int v, int d);
 
 // Parse the reference's options vector and build the geometry. dtype 0 = fp32,
 // 1 = fp64. Returns false and sets `err` on invalid options.

@@ -259,7 +259,10 @@ int ctgb_version(void);
  * 6 ramp taps (2D-1), 7 the image gather's split line maps as stored for `dtype`
  * (V*L*4: alpha hi, alpha lo, sigma hi, sigma lo, each rounded to the type; the
  * high parts make alpha_hi + sigma_hi*k exact for every pixel edge k of the
- * line). Returns the element count, or -1 on error. */
+ * line), 8 the detector gather's cell walks as stored for fp32 (V*D*6: lower
+ * boundary u0 and its step du per line in pixel-edge units, width w0 and its
+ * step dw, first and last line on which the cell meets the image, first > last
+ * for none). Returns the element count, or -1 on error. */
 long ctgb_geometry_query(const double* options, int n_options, int dtype, int what, double* out,
                          size_t n_out);
 

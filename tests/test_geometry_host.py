@@ -179,3 +179,31 @@ def test_split_line_maps_exact_high_part(native, opts, dtype):
         # rounds in double (a few units in the last place)
         tol = 2.0 ** -36 if dtype == 0 else 2.0 ** -50
         assert (np.abs(got - want).max(axis=1) <= tol * scale).all(), v
+
+
+@pytest.mark.parametrize("opts", CASES + [
+    fan_options(7, 3, 9, 5, 1.0, 9.0, 0.1, 2 * math.pi / 7, 40.0, 30.0, 0.0, FAN_ED),  # cells wider than the image
+    para_options(5, 1, 1, 1, 1.0, 0.25, 0.2, math.pi / 5, 0.0),
+])
+def test_cell_walks_match_line_maps(native, opts):
+    """Every cell's fixed-point walk gives the boundary of each line's own map
+    (to 2^-27 pixels, 2^-22 of the width), and its line range holds every line
+    on which the cell overlaps the image."""
+    V, D, W, H = (int(x) for x in opts[:4])
+    L = max(W, H)
+    flags = _query(native, opts, 0).astype(int)
+    db = _query(native, opts, 1).reshape(V, D + 1)
+    lp = _query(native, opts, 3).reshape(V, L, 2)
+    walk = _query(native, opts, 8).reshape(V, D, 6)
+    for v in range(V):
+        nl, N = (H, W) if flags[v] & 1 else (W, H)
+        l = np.arange(nl)[:, None]
+        u = (db[v][None] - lp[v, :nl, :1]) / lp[v, :nl, 1:]
+        u0, du, w0, dw, first, last = walk[v].T
+        scale = np.maximum(1, np.abs(u).max())
+        assert np.abs(u0 + du * l - u[:, :-1]).max() < 2 ** -27 + 1e-12 * scale
+        width = np.diff(u, axis=1)
+        assert (np.abs(w0 + dw * l - width) < 2 ** -22 * np.maximum(width, w0)).all()
+        meets = (u[:, 1:] > 0) & (u[:, :-1] < N)
+        assert not (meets & ((l < first) | (l > last))).any()
+        assert first.min() >= 0 and last.max() < nl

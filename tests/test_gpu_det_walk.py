@@ -1,0 +1,51 @@
+"""The fp32 detector gather's fixed-point walk at the sizes where it can go
+wrong: single pixels, lines and cells, lines one past a block of four or a fold
+of 32, rows past a multiple of 32 cells, cells much wider and much narrower than
+a pixel, cells off the image; every slices-per-thread width.
+
+Tolerance: an overlap is formed from a position good to 2^-24 pixels and a width
+good to 2^-23 of itself, a weight adds 3 roundings and at most 2 ulp of a
+reciprocal, and sums round by 2^-24 per term within blocks of 32 lines: below
+8 * 2^-23 = 9.5e-7 of the result's norm."""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from ctlib_gb300.workloads import FAN_EA, FAN_ED, fan_options, para_options
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [  # views, dets, width, height, cell width in pixels
+    (3, 1, 1, 1, 0.7), (5, 33, 4, 7, 1.1), (4, 3, 9, 5, 7.0), (6, 97, 31, 66, 0.3), (9, 64, 33, 32, 1.0),
+    (7, 40, 65, 3, 2.6), (8, 31, 2, 129, 1.6),
+]
+
+
+def _options(scan, V, D, W, H, cell, shift):
+    r = 4.0 * max(W, H, D * cell / 2) + 8
+    if scan == FAN_ED:
+        return fan_options(V, D, W, H, 1.0, 1.6 * cell, 0.2, 2 * math.pi / V, r, 0.6 * r, shift, scan)
+    if scan == FAN_EA:
+        return fan_options(V, D, W, H, 1.0, cell / r, 0.2, 2 * math.pi / V, r, 0.6 * r, shift / r, scan)
+    return para_options(V, D, W, H, 1.0, cell, 0.2, math.pi / V, shift)
+
+
+@pytest.mark.parametrize("scan", [0, 1, 2])
+@pytest.mark.parametrize("size", SIZES)
+def test_walk_edges(oracle_mod, scan, size):
+    import ctlib_gb300 as ct
+    V, D, W, H, cell = size
+    opts = _options(scan, V, D, W, H, cell, 0.35 * cell)
+    o = torch.tensor(opts, dtype=torch.float32)
+    x = np.random.default_rng(V * D + W).uniform(0.5, 1.5, (17, 1, H, W)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    for op in ("projection", "backprojection_t"):
+        f = getattr(ct, op)
+        whole = f(xd, o)
+        want = oracle_mod.run(op, x, opts, oracle_mod.MODE_F64_ON_F32)
+        assert oracle_mod.rel_l2(whole.cpu().numpy(), want) <= 8 * 2.0 ** -23, op
+        for n in (1, 2, 3, 8):  # other slices per thread: the same bits
+            assert torch.equal(f(xd[:n].contiguous(), o), whole[:n]), (op, n)
