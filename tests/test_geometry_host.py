@@ -207,3 +207,30 @@ def test_cell_walks_match_line_maps(native, opts):
         meets = (u[:, 1:] > 0) & (u[:, :-1] < N)
         assert not (meets & ((l < first) | (l > last))).any()
         assert first.min() >= 0 and last.max() < nl
+
+
+def test_cell_walks_of_rays_along_the_lines(native):
+    """A fan of almost 90 degrees: at 45 degrees its outer rays run along the
+    image lines, and their positions leave any fixed-point range. On every line
+    the stored walk is exact near the image and on the right side far from it."""
+    V, D, L = 8, 20, 128
+    for eps in (1e-8, 2e-8, 4e-8, 6e-8, 8e-8, 1e-7, 1.5e-7, 2e-7):
+        opts = fan_options(V, D, L, L, 1.0, (math.pi / 4 - eps) / 10, 0.0, math.pi / 4, 120.0, 100.0, 0.0, FAN_EA)
+        try:
+            db = _query(native, opts, 1).reshape(V, D + 1)
+        except ValueError:  # past 90 degrees once rounded to fp32
+            continue
+        break
+    lp = _query(native, opts, 3).reshape(V, L, 2)
+    walk = _query(native, opts, 8).reshape(V, D, 6)
+    l = np.arange(L)[:, None]
+    far = 0
+    for v in range(V):
+        u = (db[v][None, :-1] - lp[v, :, :1]) / lp[v, :, 1:]
+        got = walk[v, :, 0] + walk[v, :, 1] * l
+        near = np.abs(u) < 1e5
+        assert np.abs(got - u)[near].max() < 2 ** -27 + 1e-9 * np.abs(db[v]).max()
+        assert (np.abs(got[~near]) > 65536).all() and (np.sign(got) == np.sign(u))[~near].all()
+        assert np.abs(got).max() < 2.0 ** 31 - 8
+        far += (~near).sum()
+    assert far > 0

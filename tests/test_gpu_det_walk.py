@@ -49,3 +49,33 @@ def test_walk_edges(oracle_mod, scan, size):
         assert oracle_mod.rel_l2(whole.cpu().numpy(), want) <= 8 * 2.0 ** -23, op
         for n in (1, 2, 3, 8):  # other slices per thread: the same bits
             assert torch.equal(f(xd[:n].contiguous(), o), whole[:n]), (op, n)
+
+
+@pytest.mark.parametrize("scan", [0, 1, 2])
+@pytest.mark.parametrize("size", [(300, 200, 96, 80, 0.9), (64, 70, 130, 130, 2.4), (361, 33, 40, 37, 1.2)])
+def test_staged_lines_match_global_ones(scan, size):
+    """From eight slices per thread on, lines are staged in shared memory where the
+    views lie close enough; fewer read global memory. The bits
+    agree, also when every wait for a staged slot gives up at once."""
+    import ctlib_gb300 as ct
+    from ctlib_gb300 import _native as N
+    from ctlib_gb300.ops import Plan
+    V, D, W, H, cell = size
+    opts = _options(scan, V, D, W, H, cell, 0.0)
+    o = torch.tensor(opts, dtype=torch.float32)
+    g = torch.Generator().manual_seed(7)
+    x = torch.randn(21, 1, H, W, generator=g).cuda()
+    N.wait_timeouts(0, reset=True)
+    for op, name in ((0, "projection"), (3, "backprojection_t")):
+        f = getattr(ct, name)
+        one = torch.cat([f(x[i:i + 1].contiguous(), o) for i in range(21)])
+        for n in (21, 16, 7, 4):
+            assert torch.equal(f(x[:n].contiguous(), o), one[:n]), (name, n)
+        assert N.wait_timeouts(0) == 0
+        plan = Plan(tuple(opts), torch.float32, 0)
+        N.check(N.lib().ctgb_plan_set_wait_limit(plan.handle, 0), "wait limit")
+        out = torch.empty_like(one)
+        plan.run(op, x, out)
+        torch.cuda.synchronize()
+        assert torch.equal(out, one), name
+        N.wait_timeouts(0, reset=True)
