@@ -59,6 +59,13 @@ struct CellWalk {
 };
 CellWalk cell_walk(const HostGeom& g, int v, int d);
 
+// u0 and du of boundary b (0 .. D) of view v as unevaluated pairs, good to about
+// 100 bits for the boundary's axis coordinate as it is stored
+struct BoundaryWalk {
+  double u0, u0_lo, du, du_lo;
+};
+BoundaryWalk boundary_walk(const HostGeom& g, int v, int b);
+
 // Parse the reference's options vector and build the geometry. dtype 0 = fp32,
 // 1 = fp64. Returns false and sets `err` on invalid options.
 bool build_geometry(const double* options, int n_options, int dtype, HostGeom& g, std::string& err);

@@ -1,4 +1,4 @@
-"""The fp32 detector gather's fixed-point walk at the sizes where it can go
+"""The detector gather's fixed-point walk at the sizes where it can go
 wrong: single pixels, lines and cells, lines one past a block of four or a fold
 of 32, rows past a multiple of 32 cells, cells much wider and much narrower than
 a pixel, cells off the image; every slices-per-thread width.
@@ -6,7 +6,8 @@ a pixel, cells off the image; every slices-per-thread width.
 Tolerance: an overlap is formed from a position good to 2^-24 pixels and a width
 good to 2^-23 of itself, a weight adds 3 roundings and at most 2 ulp of a
 reciprocal, and sums round by 2^-24 per term within blocks of 32 lines: below
-8 * 2^-23 = 9.5e-7 of the result's norm."""
+8 * 2^-23 = 9.5e-7 of the result's norm. In fp64 the axis coordinates, up to 1e3
+pixels, are rounded by 2^-53: below 4e-13 of a cell of 0.3 pixels, so 1e-12."""
 
 import math
 
@@ -33,20 +34,23 @@ def _options(scan, V, D, W, H, cell, shift):
     return para_options(V, D, W, H, 1.0, cell, 0.2, math.pi / V, shift)
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("scan", [0, 1, 2])
 @pytest.mark.parametrize("size", SIZES)
-def test_walk_edges(oracle_mod, scan, size):
+def test_walk_edges(oracle_mod, scan, size, dtype):
     import ctlib_gb300 as ct
     V, D, W, H, cell = size
     opts = _options(scan, V, D, W, H, cell, 0.35 * cell)
-    o = torch.tensor(opts, dtype=torch.float32)
-    x = np.random.default_rng(V * D + W).uniform(0.5, 1.5, (17, 1, H, W)).astype(np.float32)
+    f32 = dtype == np.float32
+    o = torch.tensor(opts, dtype=torch.float64)
+    mode, tol = (oracle_mod.MODE_F64_ON_F32, 8 * 2.0 ** -23) if f32 else (oracle_mod.MODE_F64, 1e-12)
+    x = np.random.default_rng(V * D + W).uniform(0.5, 1.5, (17, 1, H, W)).astype(dtype)
     xd = torch.from_numpy(x).cuda()
     for op in ("projection", "backprojection_t"):
         f = getattr(ct, op)
         whole = f(xd, o)
-        want = oracle_mod.run(op, x, opts, oracle_mod.MODE_F64_ON_F32)
-        assert oracle_mod.rel_l2(whole.cpu().numpy(), want) <= 8 * 2.0 ** -23, op
+        want = oracle_mod.run(op, x, opts, mode)
+        assert oracle_mod.rel_l2(whole.cpu().numpy(), want) <= tol, op
         for n in (1, 2, 3, 8):  # other slices per thread: the same bits
             assert torch.equal(f(xd[:n].contiguous(), o), whole[:n]), (op, n)
 
