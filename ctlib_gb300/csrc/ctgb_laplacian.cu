@@ -287,10 +287,22 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 1)
         ld4s<T>(sA + kk * SA + rw, av);
         ld4s<T>(sA + kk * SA + rw + 4, av + 4);
         ld4s<T>(sB + kk * SBW + 4 * lane, bv);
+        // fp32: packed multiply-adds on pairs of rows, which lie side by side in sA
+        // (half the issue slots, the same rounding)
 #pragma unroll
-        for (int a = 0; a < 8; ++a)
+        for (int a = 0; a < 8; a += 2)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) acc[a][q] = fma(av[a], bv[q], acc[a][q]);
+          for (int q = 0; q < 4; ++q) {
+            if constexpr (sizeof(T) == 4) {
+              const float2 r = __ffma2_rn(make_float2(av[a], av[a + 1]), make_float2(bv[q], bv[q]),
+                                          make_float2(acc[a][q], acc[a + 1][q]));
+              acc[a][q] = r.x;
+              acc[a + 1][q] = r.y;
+            } else {
+              acc[a][q] = fma(av[a], bv[q], acc[a][q]);
+              acc[a + 1][q] = fma(av[a + 1], bv[q], acc[a + 1][q]);
+            }
+          }
       }
     }
     // distances; columns past the range are NaN (never selected)
