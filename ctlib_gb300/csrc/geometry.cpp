@@ -49,7 +49,7 @@ bool build(const double* o, int n, HostGeom& g, std::string& err) {
   g.db.assign((size_t)V * (D + 1), 0.0);
   g.wd.assign((size_t)V * D, 0.0);
   g.fq.assign((size_t)V * D, 0.0);
-  g.fbt.assign((size_t)V * D, 1.0);
+  if (g.scan == kFanEA) g.fbt.assign((size_t)V * D, 0.0);
   g.lp.assign((size_t)V * L * 2, 0.0);
   g.inv.assign((size_t)V * 5, 0.0);
   g.slope.assign(V, 0.0);
@@ -258,41 +258,6 @@ BoundaryWalk boundary_walk(const HostGeom& g, int v, int b) {
   Pair u = p0 * t.hi + p0 * t.lo;
   u = (u + sum(x, -edge)) / h;
   return {u.hi, u.lo, t.hi * step, t.lo * step};
-}
-
-CellWalk cell_walk(const HostGeom& g, int v, int d) {
-  const bool xb = g.flags[v] & 1;
-  const int nl = xb ? g.H : g.W, N = xb ? g.W : g.H;
-  const double h = g.dImg, edge = xb ? g.x0 : g.y0;
-  // line l lies at p0 + l * step across the walk (rows go down, columns right)
-  const double p0 = xb ? (g.height / 2 - 0.5) * h : (0.5 - g.width / 2) * h, step = xb ? -1.0 : 1.0;
-  const double across = xb ? g.src[2 * v + 1] : g.src[2 * v], along = xb ? g.src[2 * v] : g.src[2 * v + 1];
-  auto ray = [&](double b, double& u0, double& du) {
-    // position along the walk at line position p: b + t p with t = (along - b) /
-    // across for a fan's ray through the source, -slope for a parallel one
-    const double t = g.scan == kPara ? -g.slope[v] : (along - b) / across;
-    u0 = (b + t * p0 - edge) / h;
-    du = t * step;
-  };
-  CellWalk c;
-  double u1, du1;
-  const size_t b = (size_t)v * (g.D + 1) + d;
-  ray(g.db[b], c.u0, c.du);
-  ray(g.db[b + 1], u1, du1);
-  c.w0 = u1 - c.u0;
-  c.dw = du1 - c.du;
-  double lo = 0, hi = nl - 1;
-  // lines with a + s l > 0
-  auto keep = [&](double a, double s) {
-    if (s > 0) lo = std::fmax(lo, std::floor(-a / s) - 1);
-    else if (s < 0) hi = std::fmin(hi, std::ceil(-a / s) + 1);
-    else if (!(a > 0)) hi = -1;
-  };
-  keep(u1, du1);         // the upper boundary right of the image's left edge
-  keep(N - c.u0, -c.du); // the lower boundary left of its right edge
-  if (lo <= hi) { c.first = (int)lo; c.last = (int)hi; }
-  else { c.first = 65535; c.last = 0; }
-  return c;
 }
 
 // RL kernel value at integer offset x for tap spacing d (src/fan_ed_kernel.cu:926-943)

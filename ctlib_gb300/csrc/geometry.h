@@ -16,6 +16,7 @@
 // axis = alpha + sigma * k, evaluated in fp64 from the rounded source position.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -34,7 +35,7 @@ struct HostGeom {
   std::vector<double> db;      // V*(D+1): cell boundaries on the axis, increasing
   std::vector<double> wd;      // V*D: cell widths db[d+1]-db[d]
   std::vector<double> fq;      // V*D: A / A^T factor (fan dImg/(cbar*w), para dImg/dDet)
-  std::vector<double> fbt;     // V*D: extra B^T factor (EA: dImg/cbar), 1 otherwise
+  std::vector<double> fbt;     // V*D: B^T factor of equal-angle fans (dImg/cbar), empty otherwise
   std::vector<double> lp;      // V*L*2: alpha, sigma (pixel edge k of a line maps to alpha + sigma*k)
   std::vector<double> inv;     // V*5: guess u = x*P0/(P1+x*P2) (atan for EA), cell = P3+P4*u
   std::vector<double> wpre;    // D: fbp detector pre-weight, applied as (y * wpre[k]) * wscale
@@ -50,6 +51,9 @@ struct HostGeom {
 // A detector-cell boundary is a straight ray, so its position on the image
 // lines of a view, in pixel-edge units, is linear in the line index: u(l) = u0 +
 // du * l. Likewise the cell's width w(l) = w0 + dw * l in pixels.
+struct RayWalk {
+  double u0, du;
+};
 struct CellWalk {
   double u0, du;  // lower boundary
   double w0, dw;  // width
@@ -57,7 +61,43 @@ struct CellWalk {
   // the image (one line of margin on each side); first > last: none
   int first, last;
 };
-CellWalk cell_walk(const HostGeom& g, int v, int d);
+
+// boundary b (0 .. D) of view v
+inline RayWalk ray_walk(const HostGeom& g, int v, int b) {
+  const bool xb = g.flags[v] & 1;
+  const double h = g.dImg, edge = xb ? g.x0 : g.y0;
+  // line l lies at p0 + l * step across the walk (rows go down, columns right)
+  const double p0 = xb ? (g.height / 2 - 0.5) * h : (0.5 - g.width / 2) * h, step = xb ? -1.0 : 1.0;
+  const double across = xb ? g.src[2 * v + 1] : g.src[2 * v], along = xb ? g.src[2 * v] : g.src[2 * v + 1];
+  // position along the walk at line position p: x + t p with t = (along - x) /
+  // across for a fan's ray through the source, -slope for a parallel one
+  const double x = g.db[(size_t)v * (g.D + 1) + b];
+  const double t = g.scan == kPara ? -g.slope[v] : (along - x) / across;
+  return {(x + t * p0 - edge) / h, t * step};
+}
+
+// the cell between two boundaries
+inline CellWalk cell_walk(const HostGeom& g, int v, RayWalk lower, RayWalk upper) {
+  const bool xb = g.flags[v] & 1;
+  const int nl = xb ? g.H : g.W, N = xb ? g.W : g.H;
+  CellWalk c;
+  c.u0 = lower.u0;
+  c.du = lower.du;
+  c.w0 = upper.u0 - lower.u0;
+  c.dw = upper.du - lower.du;
+  double lo = 0, hi = nl - 1;
+  // lines with a + s l > 0
+  auto keep = [&](double a, double s) {
+    if (s > 0) lo = std::fmax(lo, std::floor(-a / s) - 1);
+    else if (s < 0) hi = std::fmin(hi, std::ceil(-a / s) + 1);
+    else if (!(a > 0)) hi = -1;
+  };
+  keep(upper.u0, upper.du);  // the upper boundary right of the image's left edge
+  keep(N - c.u0, -c.du);     // the lower boundary left of its right edge
+  if (lo <= hi) { c.first = (int)lo; c.last = (int)hi; }
+  else { c.first = 65535; c.last = 0; }
+  return c;
+}
 
 // u0 and du of boundary b (0 .. D) of view v as unevaluated pairs, good to about
 // 100 bits for the boundary's axis coordinate as it is stored
