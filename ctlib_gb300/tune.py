@@ -5,9 +5,9 @@ for one operator on one plan (`ctgb_plan_set_schedule`, `ctgb_plan_set_unroll`).
 Carrying more slices per thread amortises the per-(view, line) geometry over
 more fused multiply-adds but costs registers and therefore resident warps;
 fewer warps per CTA changes how views (detector gather) or image rows (image
-gather) are grouped; two straight-line steps instead of three skip the third
-pixel (cell) that most cells (pixels) do not reach, at the price of a
-divergent remainder loop where some do. The best choice depends on the
+gather) are grouped; two straight-line steps instead of three, a choice of the
+fp32 image gather at one or two slices per thread, skip the third cell that most
+pixels do not reach, at the price of a divergent remainder loop where some do. The best choice depends on the
 geometry, the batch and the GPU, so it is measured: every
 candidate is timed with CUDA events on the caller's device and the fastest is
 kept, in memory and in a JSON cache on disk

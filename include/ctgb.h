@@ -72,14 +72,15 @@ int ctgb_plan_set_schedule(ctgb_plan* plan, int op, int slices_per_thread, int w
  * picked from the geometry): the overlapped cells per pixel (projection_t,
  * backprojection, fbp, backprojection_sv) evaluated without a branch before a
  * remainder loop takes any further ones. Both are built for one and two fp32
- * slices per thread; more take 2 and fp64 takes 3, whatever is set, and
- * projection and backprojection_t follow the cell widths line by line.
- * Results do not depend on it. No counterpart
- * in the reference (its merge walk has no fixed step count). */
+ * slices per thread; more, and fp64, take 2 whatever is set, and projection and
+ * backprojection_t follow the cell widths line by line. Results do not depend
+ * on it. No counterpart in the reference (its merge walk has no fixed step
+ * count). */
 int ctgb_plan_set_unroll(ctgb_plan* plan, int op, int steps);
 
-/* Limit, in nanoseconds, of every bounded wait in the staged image gather
- * (projection_t, backprojection, fbp, backprojection_sv) on this plan:
+/* Limit, in nanoseconds, of every bounded wait on this plan, in the staged image
+ * gather (projection_t, backprojection, fbp, backprojection_sv) and the staged
+ * detector gather (projection and backprojection_t of 8 slices or more):
  * 1000000000 (1 s) by default, at most 10 s. A wait that runs out makes its
  * CTA finish on global loads, with the same results, and is counted by
  * ctgb_wait_timeouts. 0 makes every wait give up unless its copy has already
@@ -192,10 +193,11 @@ int ctgb_data_gradient(const ctgb_plan* plan, const void* image, const void* sin
  * stall other streams; a reconstruction service that reserves all of its
  * device memory at start-up treats a later allocation as a fault. This entry
  * point takes only the input and output buffers and uses instead a fixed
- * static scratch array of ctgb_projection_noalloc_max_bytes() bytes (64 MiB)
- * inside this library, reserved on every GPU that loads it until process exit.
- * A batch whose scratch (ctgb_workspace_size for CTGB_OP_PROJECTION) exceeds
- * that size fails with CTGB_ERR_WORKSPACE. The first call on a device (and the
+ * static scratch array inside this library (72 MiB), reserved on every GPU that
+ * loads it until process exit. A batch whose image lines, without the padding of
+ * a few pixels per line that ctgb_workspace_size counts, take more than
+ * ctgb_projection_noalloc_max_bytes() bytes (64 MiB) fails with
+ * CTGB_ERR_WORKSPACE. The first call on a device (and the
  * first after its context is destroyed and created again, e.g. by
  * cudaDeviceReset) looks up the array's device address; make that first call
  * before any stream capture. All calls share the one array, which keeps the
@@ -204,7 +206,7 @@ int ctgb_data_gradient(const ctgb_plan* plan, const void* image, const void* sin
  * must be serialised by the caller. */
 int ctgb_projection_noalloc(const ctgb_plan* plan, const void* image, void* sino, int batch, void* stream);
 
-/* Size in bytes of the static scratch array used by ctgb_projection_noalloc. */
+/* Bytes of image lines that ctgb_projection_noalloc takes at most. */
 size_t ctgb_projection_noalloc_max_bytes(void);
 
 /* Ragged batches: n slices (1..128), each with its own plan (image size, views,
