@@ -577,7 +577,7 @@ def run_ours(args):
     ta, tat = statistics.mean(t_a), statistics.mean(t_at)
     ka, kat = _kernel_times(plan, args.steps, flush, stream, lambda: ctlib.projection(img, opts),
                             lambda s: ctlib.projection_t(s, opts))
-    dom = "k_det_gather (projection)" if ka >= kat else "k_pix_gather (projection_t)"
+    dom = "detector_gather (projection)" if ka >= kat else "image_gather (projection_t)"
     dom_ms = max(ka, kat)
     # algorithmic bytes of one launch: read input + write output once
     alg_bytes = (B * H * W + B * V * D) * 4
@@ -622,7 +622,7 @@ def run_ours(args):
                           "note": "one projection + projection_t call per slice"},
                 "batched_over_plain": value / ws / plain_value,
                 "ms_projection": ta, "ms_projection_t": tat,
-                "kernel_ms": {"k_det_gather": ka, "k_pix_gather": kat},
+                "kernel_ms": {"detector_gather": ka, "image_gather": kat},
                 "e2e": {"value": e2e_value, "unit": UNIT, "ms_per_step": e2e_mean,
                         "h2d_bytes_per_step": int(img_h.numel() * 4),
                         "d2h_bytes_per_step": int(img_h.numel() * 4 + 4),
