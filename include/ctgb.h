@@ -265,7 +265,10 @@ int ctgb_version(void);
  * line), 8 the detector gather's cell walks as stored for fp32 (V*D*6: lower
  * boundary u0 and its step du per line in pixel-edge units, width w0 and its
  * step dw, first and last line on which the cell meets the image, first > last
- * for none). Returns the element count, or -1 on error. */
+ * for none), 9 the fp64 image gather's line maps as stored (V*L*7: high and low 32
+ * bits of alpha and of sigma, whole units of 2^-s; 32 more bits of sigma, signed,
+ * and of alpha; s. Pixel edge k is alpha + sigma*k + ((alpha_lo + sigma_lo*k) >>
+ * 32)). Returns the element count, or -1 on error. */
 long ctgb_geometry_query(const double* options, int n_options, int dtype, int what, double* out,
                          size_t n_out);
 

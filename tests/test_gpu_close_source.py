@@ -39,3 +39,18 @@ def test_detector_gather(oracle_mod, op, scan, ratio):
     want = oracle_mod.run(op, x, opts, oracle_mod.MODE_F64_ON_F32)
     for v in range(144):  # view by view: only those with the source below or right of the image can fail
         assert oracle_mod.rel_l2(got[:, :, v].cpu().numpy(), want[:, :, v]) <= 8 * 2.0 ** -23, v
+
+
+@pytest.mark.parametrize("op", ["projection_t", "backprojection", "projection", "backprojection_t"])
+@pytest.mark.parametrize("scan", [FAN_ED, FAN_EA])
+@pytest.mark.parametrize("ratio", [0.8, 0.72])
+def test_double_precision(oracle_mod, op, scan, ratio):
+    """Pixels next to the source take more than 52 bits of the image gather's units.
+    Axis coordinates of up to 2^8 pixels, off by 4 roundings of 2^-53: 1e-12 of a
+    pixel of 0.5 on the far side holds 4 times over."""
+    import ctlib_gb300 as ct
+    opts = _options(scan, ratio, 256, 24, 368)
+    image = op in ("projection", "backprojection_t")
+    x = np.random.default_rng(4).standard_normal((3, 1) + ((256, 256) if image else (24, 368)))
+    got = getattr(ct, op)(torch.from_numpy(x).cuda(), torch.tensor(opts, dtype=torch.float64)).cpu().numpy()
+    assert oracle_mod.rel_l2(got, oracle_mod.run(op, x, opts, oracle_mod.MODE_F64)) <= 1e-12
