@@ -14,7 +14,7 @@ import numpy as np
 import pytest
 import torch
 
-from ctlib_gb300.workloads import FAN_ED, fan_options, para_options
+from ctlib_gb300.workloads import FAN_EA, FAN_ED, fan_options, para_options
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +59,50 @@ def test_fan_weights_are_rounded_reciprocals():
     got = ct.backprojection(torch.ones(1, 1, 1, 1, device="cuda"), o).cpu().numpy()[0, 0]
     want = length * (np.float32(1) / (t2 * length))
     assert (got == want[:, None]).all()
+
+
+U64 = 2.0 ** -53
+
+
+@pytest.mark.parametrize("scan", [FAN_ED, FAN_EA])
+@pytest.mark.parametrize("col", range(6))
+def test_double_overlaps_are_divided_to_a_few_ulp(scan, col):
+    """B^T in fp64 of one pixel of 1 that a wide cell covers, at every place of the
+    walk's two straight pixels and its remainder. Roundings: the product of two
+    divisors, its reciprocal (one, and below 2^-57 of the method) and the factor
+    back, 3; squared, 6, the square and the overlap's product 2: 8 and a little.
+    Equal-angle fans: 4 so far, 3 of the distance, 2 of the cell's factor and its
+    product, whose table adds up to 5: 14."""
+    import ctlib_gb300 as ct
+    H, W, r = 256, 6, 1024.0
+    L = np.longdouble
+    d = 8.0 * W if scan == FAN_ED else 0.05
+    opts = fan_options(1, 1, W, H, 1.0, d, 0.0, 2 * math.pi, r, r, 0.0, scan)
+    x = torch.zeros(H, 1, H, W, dtype=torch.float64)
+    x[torch.arange(H), 0, torch.arange(H), col] = 1
+    got = ct.backprojection_t(x.cuda(), torch.tensor(opts, dtype=torch.float64)).cpu().numpy().ravel().astype(L)
+    y = H / 2 - np.arange(H).astype(L) - L(0.5)
+    if scan == FAN_ED:
+        want, tol = 1 / (1 - y / r) ** 2, 9 * U64
+    else:
+        cbar = np.cos(L(d) / 2)  # both boundaries alike
+        want, tol = 1 / ((L(col) + L(0.5) - L(W) / 2) ** 2 + (r - y) ** 2) / cbar, 14 * U64
+    assert (np.abs(got / want - 1) <= tol).all(), float(np.abs(got / want - 1).max() / U64)
+
+
+@pytest.mark.parametrize("scan", [FAN_ED, FAN_EA])
+def test_double_weights_are_good_to_a_few_ulp(scan):
+    """B in fp64 of one wide cell of 1: the pixel's length, an integer of 2^50 units
+    or more (4 U64 at its worst), times the weight (its divisor 4, reciprocal and
+    product 3), to the unit and back 1: 12."""
+    import ctlib_gb300 as ct
+    H, W, r = 256, 6, 1024.0
+    L = np.longdouble
+    d = 8.0 * W if scan == FAN_ED else 0.05
+    opts = fan_options(1, 1, W, H, 1.0, d, 0.0, 2 * math.pi, r, r, 0.0, scan)
+    got = ct.backprojection(torch.ones(1, 1, 1, 1, dtype=torch.float64, device="cuda"),
+                            torch.tensor(opts, dtype=torch.float64)).cpu().numpy()[0, 0].astype(L)
+    y = (H / 2 - np.arange(H).astype(L) - L(0.5))[:, None]
+    q = np.arange(W).astype(L) + L(0.5) - L(W) / 2
+    want = 1 / (1 - y / r) ** 2 + 0 * q if scan == FAN_ED else 1 / (q ** 2 + (r - y) ** 2)
+    assert (np.abs(got / want - 1) <= 12 * U64).all(), float(np.abs(got / want - 1).max() / U64)
