@@ -613,8 +613,8 @@ int run(const T* x, int n, int dim, int k, long long* ind, float* val, unsigned 
   if (smem > (size_t)optin)
     return fail(CTGB_ERR_INVALID, "laplacian: k too large for this dtype (" + std::to_string(smem) +
                                       " bytes of shared memory per CTA needed)");
-  e = cudaFuncSetAttribute(k_knn<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_knn<T>, NT, smem);
+  if (const int rc = allow_smem((const void*)k_knn<T>, optin, "laplacian")) return rc;  // (no static shared memory)
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_knn<T>, NT, smem);
   if (e != cudaSuccess) return fail(CTGB_ERR_CUDA, std::string("laplacian smem: ") + cudaGetErrorString(e));
   const int ns = choose_split(n, L.max_split, sms * std::max(1, occ));
   const int cps = ((n + ns - 1) / ns + TN - 1) / TN * TN;
