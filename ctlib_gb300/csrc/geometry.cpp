@@ -217,47 +217,21 @@ bool build(const double* o, int n, HostGeom& g, std::string& err) {
 
 }  // namespace
 
-namespace {
-
-// Unevaluated sums of two doubles (T. J. Dekker, "A floating-point technique for
-// extending the available precision", 1971), with fused multiply-adds for the
-// products' errors.
-struct Pair {
-  double hi, lo;
-};
-Pair fast_sum(double a, double b) {
-  const double s = a + b;
-  return {s, b - (s - a)};
-}
-Pair sum(double a, double b) {
-  const double s = a + b, t = s - a;
-  return {s, (a - (s - t)) + (b - t)};
-}
-Pair operator+(Pair a, Pair b) {
-  const Pair s = sum(a.hi, b.hi);
-  return fast_sum(s.hi, s.lo + a.lo + b.lo);
-}
-Pair operator*(Pair a, double b) {
-  const double p = a.hi * b;
-  return fast_sum(p, std::fma(a.hi, b, -p) + a.lo * b);
-}
-Pair operator/(Pair a, double b) {
-  const double q = a.hi / b;
-  return fast_sum(q, (std::fma(-q, b, a.hi) + a.lo) / b);
-}
-
-}  // namespace
-
-BoundaryWalk boundary_walk(const HostGeom& g, int v, int b) {
+ViewWalk view_walk(const HostGeom& g, int v) {
   const bool xb = g.flags[v] & 1;
+  const int N = xb ? g.W : g.H;
   const double h = g.dImg, edge = xb ? g.x0 : g.y0, step = xb ? -1.0 : 1.0;
   const Pair p0 = Pair{xb ? g.height / 2 - 0.5 : 0.5 - g.width / 2, 0.0} * h;  // exact factor, rounded product
+  // position on line l = (x + t (p0 + step h l) - edge) / h for the boundary at x, of slope t
+  if (g.scan == kPara) {
+    const double t = -g.slope[v];
+    return {Pair{1.0, 0.0} / h, (p0 * t + Pair{-edge, 0.0}) / h, {0.0, 0.0}, {t * step, 0.0}, N};
+  }
+  // t = (along - x) / across
   const double across = xb ? g.src[2 * v + 1] : g.src[2 * v], along = xb ? g.src[2 * v] : g.src[2 * v + 1];
-  const double x = g.db[(size_t)v * (g.D + 1) + b];
-  const Pair t = g.scan == kPara ? Pair{-g.slope[v], 0.0} : sum(along, -x) / across;
-  Pair u = p0 * t.hi + p0 * t.lo;
-  u = (u + sum(x, -edge)) / h;
-  return {u.hi, u.lo, t.hi * step, t.lo * step};
+  const Pair q = p0 / across;
+  return {(Pair{1.0, 0.0} + Pair{-q.hi, -q.lo}) / h, (q * along + Pair{-edge, 0.0}) / h, Pair{-step, 0.0} / across,
+          Pair{step * along, 0.0} / across, N};
 }
 
 // RL kernel value at integer offset x for tap spacing d (src/fan_ed_kernel.cu:926-943)

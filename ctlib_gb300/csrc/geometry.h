@@ -53,7 +53,12 @@ struct HostGeom {
 // du * l. Likewise the cell's width w(l) = w0 + dw * l in pixels.
 struct RayWalk {
   double u0, du;
+  double left, right;  // the (fractional) lines on which u is 0 and N; nothing if du is 0
 };
+inline RayWalk ray_walk(double u0, double du, int N) {
+  const double r = 1 / du;
+  return {u0, du, -u0 * r, (N - u0) * r};
+}
 struct CellWalk {
   double u0, du;  // lower boundary
   double w0, dw;  // width
@@ -61,20 +66,6 @@ struct CellWalk {
   // the image (one line of margin on each side); first > last: none
   int first, last;
 };
-
-// boundary b (0 .. D) of view v
-inline RayWalk ray_walk(const HostGeom& g, int v, int b) {
-  const bool xb = g.flags[v] & 1;
-  const double h = g.dImg, edge = xb ? g.x0 : g.y0;
-  // line l lies at p0 + l * step across the walk (rows go down, columns right)
-  const double p0 = xb ? (g.height / 2 - 0.5) * h : (0.5 - g.width / 2) * h, step = xb ? -1.0 : 1.0;
-  const double across = xb ? g.src[2 * v + 1] : g.src[2 * v], along = xb ? g.src[2 * v] : g.src[2 * v + 1];
-  // position along the walk at line position p: x + t p with t = (along - x) /
-  // across for a fan's ray through the source, -slope for a parallel one
-  const double x = g.db[(size_t)v * (g.D + 1) + b];
-  const double t = g.scan == kPara ? -g.slope[v] : (along - x) / across;
-  return {(x + t * p0 - edge) / h, t * step};
-}
 
 // the cell between two boundaries
 inline CellWalk cell_walk(const HostGeom& g, int v, RayWalk lower, RayWalk upper) {
@@ -86,25 +77,60 @@ inline CellWalk cell_walk(const HostGeom& g, int v, RayWalk lower, RayWalk upper
   c.w0 = upper.u0 - lower.u0;
   c.dw = upper.du - lower.du;
   double lo = 0, hi = nl - 1;
-  // lines with a + s l > 0
-  auto keep = [&](double a, double s) {
-    if (s > 0) lo = std::fmax(lo, std::floor(-a / s) - 1);
-    else if (s < 0) hi = std::fmin(hi, std::ceil(-a / s) + 1);
+  // the lines on one side of where a boundary crosses an edge; a: its side if it runs along the lines
+  auto keep = [&](double a, double s, double at) {
+    if (s > 0) lo = std::fmax(lo, std::floor(at) - 1);
+    else if (s < 0) hi = std::fmin(hi, std::ceil(at) + 1);
     else if (!(a > 0)) hi = -1;
   };
-  keep(upper.u0, upper.du);  // the upper boundary right of the image's left edge
-  keep(N - c.u0, -c.du);     // the lower boundary left of its right edge
+  keep(upper.u0, upper.du, upper.left);  // the upper boundary right of the image's left edge
+  keep(N - c.u0, -c.du, lower.right);    // the lower boundary left of its right edge
   if (lo <= hi) { c.first = (int)lo; c.last = (int)hi; }
   else { c.first = 65535; c.last = 0; }
   return c;
 }
 
-// u0 and du of boundary b (0 .. D) of view v as unevaluated pairs, good to about
-// 100 bits for the boundary's axis coordinate as it is stored
+// Unevaluated sums of two doubles (T. J. Dekker, "A floating-point technique for
+// extending the available precision", 1971), with fused multiply-adds for the
+// products' errors.
+struct Pair {
+  double hi, lo;
+};
+inline Pair fast_sum(double a, double b) {
+  const double s = a + b;
+  return {s, b - (s - a)};
+}
+inline Pair operator+(Pair a, Pair b) {
+  const double s = a.hi + b.hi, t = s - a.hi;
+  return fast_sum(s, (a.hi - (s - t)) + (b.hi - t) + a.lo + b.lo);
+}
+inline Pair operator*(Pair a, double b) {
+  const double p = a.hi * b;
+  return fast_sum(p, std::fma(a.hi, b, -p) + a.lo * b);
+}
+inline Pair operator/(Pair a, double b) {
+  const double q = a.hi / b;
+  return fast_sum(q, (std::fma(-q, b, a.hi) + a.lo) / b);
+}
+
+// u0 and du of a boundary at axis coordinate x as unevaluated pairs, good to about 100
+// bits for x as it is stored. Both are linear in x, with a view's constants that hold
+// all divisions: 2.5 ms for the 850 thousand boundaries of 1152 views of 736 bins,
+// where dividing at every boundary took 16.5.
 struct BoundaryWalk {
   double u0, u0_lo, du, du_lo;
 };
-BoundaryWalk boundary_walk(const HostGeom& g, int v, int b);
+struct ViewWalk {
+  Pair a, b, c, d;  // u0 = a x + b, du = c x + d
+  int N;            // pixels of a line
+  BoundaryWalk at(double x) const {
+    const Pair u = a * x + b, s = c * x + d;
+    return {u.hi, u.lo, s.hi, s.lo};
+  }
+  // the same in plain double
+  RayWalk ray(double x) const { return ray_walk(a.hi * x + b.hi, c.hi * x + d.hi, N); }
+};
+ViewWalk view_walk(const HostGeom& g, int v);
 
 // Parse the reference's options vector and build the geometry. dtype 0 = fp32,
 // 1 = fp64. Returns false and sets `err` on invalid options.
