@@ -11,7 +11,9 @@ pixels do not reach, at the price of a divergent remainder loop where some do. T
 geometry, the batch and the GPU, so it is measured: every
 candidate is timed with CUDA events on the caller's device and the fastest is
 kept, in memory and in a JSON cache on disk
-(``$CTLIB_GB300_TUNE_CACHE``, default ``~/.cache/ctlib_gb300/tune.json``).
+(``$CTLIB_GB300_TUNE_CACHE``, default ``~/.cache/ctlib_gb300/tune.json``), where
+an entry counts for the kernels it was measured on only: its key holds a digest
+of their sources.
 
 ``ops`` applies a cached schedule automatically; ``tune()`` measures (set
 ``CTLIB_GB300_AUTOTUNE=1`` to tune every new (plan, op, batch) on first use).
@@ -25,6 +27,8 @@ batch's signature (every slice's options, the dtype, the operator chain).
 
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 import threading
@@ -33,8 +37,8 @@ import torch
 
 from . import _native as N
 
-CANDIDATES_F32 = ((16, 8, 3), (16, 8, 2), (16, 4, 3), (16, 4, 2), (8, 8, 3), (8, 8, 2), (8, 4, 2), (4, 8, 2))
-CANDIDATES_F64 = ((4, 8, 3), (4, 4, 3), (2, 8, 3))
+CANDIDATES_F32 = ((16, 8, 0), (16, 4, 0), (8, 8, 0), (8, 4, 0), (4, 8, 0))
+CANDIDATES_F64 = ((4, 8, 0), (4, 4, 0), (2, 8, 0))
 
 _lock = threading.Lock()
 _cache = None
@@ -68,9 +72,35 @@ def _save():
         pass
 
 
+@functools.lru_cache(maxsize=1)
+def _kernels() -> str:
+    """Digest of the kernels' sources (of the library, where only that is installed)."""
+    paths = N.SOURCES + N.HEADERS
+    h = hashlib.sha1()
+    for path in paths if all(map(os.path.exists, paths)) else [N.SO_PATH]:
+        with open(path, "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()[:16]
+
+
+def schedules(dtype: torch.dtype, op: int, batch: int) -> tuple:
+    """The schedules that differ for ``batch`` slices: caps of slices per thread
+    above the batch are one schedule, and the step count is a choice of the fp32
+    image gather at one and two slices per thread only."""
+    out = []
+    for cap, warps, _ in CANDIDATES_F32 if dtype == torch.float32 else CANDIDATES_F64:
+        sb = 1
+        while sb < batch and sb < cap:
+            sb *= 2
+        image = op not in (N.OP_PROJECTION, N.OP_BACKPROJECTION_T)
+        steps = (2, 3) if dtype == torch.float32 and image and sb <= 2 else (0,)
+        out += [s for s in ((sb, warps, u) for u in steps) if s not in out]
+    return tuple(out)
+
+
 def _key(plan, op: int, batch: int) -> str:
     name = torch.cuda.get_device_name(plan.device)
-    return f"{name}|{plan.dtype}|{op}|{batch}|{','.join(repr(v) for v in plan.values)}"
+    return f"{_kernels()}|{name}|{plan.dtype}|{op}|{batch}|{','.join(repr(v) for v in plan.values)}"
 
 
 def _set(plan, op: int, sb: int, warps: int, unroll: int = 0):
@@ -92,8 +122,6 @@ def apply_cached(plan, op: int, batch: int) -> bool:
         if hit is None and os.environ.get("CTLIB_GB300_AUTOTUNE") == "1":
             tune(plan, op, batch)
             hit = memo[(op, batch)]
-        if hit is not None and len(hit) == 3:  # older cache entry: (sb, warps, ms)
-            hit = [hit[0], hit[1], 0, hit[2]]
         memo[(op, batch)] = None if hit is None else (int(hit[0]), int(hit[1]), int(hit[2]))
     sched = memo[(op, batch)]
     _set(plan, op, *(sched if sched is not None else (0, 0, 0)))
@@ -115,7 +143,7 @@ def _inputs(plan, op: int, batch: int):
 def tune(plan, op: int, batch: int, reps: int = 3, candidates=None) -> dict:
     """Time every candidate schedule of `op` for `batch` slices, keep the best."""
     if candidates is None:
-        candidates = CANDIDATES_F32 if plan.dtype == torch.float32 else CANDIDATES_F64
+        candidates = schedules(plan.dtype, op, batch)
     x, out = _inputs(plan, op, batch)
     stream = torch.cuda.current_stream(x.device)
     results = []
@@ -146,10 +174,9 @@ RAGGED_CANDIDATES = (0, 1, 2, 4, 8)
 
 
 def _ragged_key(rb, ops) -> str:
-    import hashlib
     name = torch.cuda.get_device_name(rb.device)
     sig = repr((tuple(tuple(p.values) for p in rb.plans), str(rb.dtype), tuple(ops)))
-    return f"ragged|{name}|{hashlib.sha1(sig.encode()).hexdigest()}"
+    return f"ragged|{_kernels()}|{name}|{hashlib.sha1(sig.encode()).hexdigest()}"
 
 
 def ragged_cached(rb, ops):
