@@ -63,7 +63,11 @@ int ctgb_plan_info(const ctgb_plan* plan, int* views, int* dets, int* width, int
 /* Schedule of one operator on a plan, as picked by the autotuner
  * (ctlib_gb300/tune.py): the largest number of batch slices one thread carries
  * (1, 2, 4, 8, 16; 0 = default: 16 for fp32, 4 for fp64) and the warps per CTA
- * of the gather kernel (4 or 8; 0 = default 8). Changes the workspace size.
+ * of the gather kernel (4 or 8; 0 = default 8). Changes the workspace size, and
+ * no bit of the results, as the batch does not, as long as all samples are finite.
+ * An infinite or NaN sample reaches every result that overlaps it and, where steps
+ * past a cell (pixel) multiply the next samples by 0, some up to two pixels (cells)
+ * past it; which of those may depend on the slices per thread and on the steps.
  * No counterpart in the reference (its launch shape is fixed, 256 threads per
  * (slice, view, 256-bin block), src/fan_ed_kernel.cu:1179-1185). */
 int ctgb_plan_set_schedule(ctgb_plan* plan, int op, int slices_per_thread, int warps_per_cta);
@@ -73,8 +77,8 @@ int ctgb_plan_set_schedule(ctgb_plan* plan, int op, int slices_per_thread, int w
  * backprojection, fbp, backprojection_sv) evaluated without a branch before a
  * remainder loop takes any further ones. Both are built for one and two fp32
  * slices per thread; more, and fp64, take 2 whatever is set, and projection and
- * backprojection_t follow the cell widths line by line. Results do not depend
- * on it. No counterpart in the reference (its merge walk has no fixed step
+ * backprojection_t follow the cell widths line by line. Results on finite samples
+ * do not depend on it. No counterpart in the reference (its merge walk has no fixed step
  * count). */
 int ctgb_plan_set_unroll(ctgb_plan* plan, int op, int steps);
 
