@@ -164,7 +164,7 @@ EXPORTED = ("ctgb_plan_create", "ctgb_plan_destroy", "ctgb_plan_info", "ctgb_pla
 
 
 def wait_timeouts(device: int = 0, reset: bool = False) -> int:
-    """Bounded waits of the staged image gather that ran out on `device`
+    """Bounded waits of the staged gathers that ran out on `device`
     (ctgb_wait_timeouts); 0 unless a copy pipeline stalled."""
     n = ctypes.c_ulonglong(0)
     check(lib().ctgb_wait_timeouts(int(device), ctypes.byref(n), int(bool(reset))), "wait counter")

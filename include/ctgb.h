@@ -101,8 +101,8 @@ int ctgb_plan_set_wait_limit(ctgb_plan* plan, unsigned long long limit_ns);
  * into an fp32 value). The plain form exists to measure what compensation
  * buys: float32 plans only (CTGB_ERR_INVALID for float64), applied by the five
  * operators (ctgb_data_gradient and ragged batches always compensate), with
- * three straight-line steps whatever the schedule. Results of either form do
- * not depend on the schedule. No counterpart in the reference. */
+ * two straight-line cells in the image gather whatever the schedule. Results of
+ * either form do not depend on the schedule. No counterpart in the reference. */
 int ctgb_plan_set_summation(ctgb_plan* plan, int compensated);
 
 /* Ramp filter of fbp on this plan: window 0 = Ram-Lak (the reference's kernel,
